@@ -212,6 +212,29 @@ def test_flash_bwd(ops, B, S, nkv, g, d):
     close(fused, T.rope_bwd_(dqkv0.clone(), tab, S, nkv, g, d), 3e-2, 3e-2)
 
 
+@pytest.mark.parametrize("B,S,nkv,g,d", [(1, 640, 1, 4, 64), (8, 1152, 8, 1, 64), (4, 1024, 8, 3, 64), (6, 896, 4, 2, 64),
+                                         (1, 640, 1, 4, 128), (8, 1152, 8, 1, 128), (4, 1024, 8, 3, 128), (6, 896, 4, 2, 128)])
+def test_flash_fwd_work_items_and_growing_maxima(ops, B, S, nkv, g, d):
+    """Every way the forward splits a call into work items (one tile; two heads; two consecutive tiles, an even and an odd number
+    of them), several items per CTA, and keys that grow along the sequence, so that the running maximum moves in every block
+    and O is rescaled all the way."""
+    from forge_train_harness_b200.ops.cuda_ops import check_status
+    torch.manual_seed(S + g)
+    qkv = rnd(B * S, nkv * (g + 2) * d)
+    v = qkv.view(B, S, nkv, g + 2, d)
+    v[:, :, :, g] *= torch.linspace(0.5, 12.0, S, device="cuda", dtype=torch.bfloat16).view(1, S, 1, 1)
+    out, lse = ops.attention_fwd(qkv, S, nkv, g, d)
+    out2, lse2 = ops.attention_fwd(qkv, S, nkv, g, d)
+    torch.cuda.synchronize()
+    check_status()
+    assert torch.equal(out, out2) and torch.equal(lse, lse2)
+    out0, lse0 = T.attention_fwd(qkv.float(), S, nkv, g, d)
+    # out is a convex combination of V rows: P rounded to bf16 (2^-9 of each weight) and the result rounded to bf16
+    assert float((out.float() - out0).abs().max()) <= 2 * 2.0 ** -8 * float(v[:, :, :, g + 1].abs().max())
+    # lse of fp32 scores: exp2 and fp32 sums of up to S terms
+    assert float((lse - lse0).abs().max()) <= 1e-5 * float(lse0.abs().max()) + 1e-4
+
+
 def test_gemm_repeated_calls_and_views(ops):
     """Operands that are strided row views (unit inner stride) and repeated in-place updates."""
     big = rnd(512, 2048, scale=0.5)
