@@ -38,26 +38,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // the query heads of a KV group, i.e. over CTAs) use the same path.  A finalize kernel rounds that image to bf16.
 // =====================================================================================================================
 
-constexpr int kBwd64Threads = 448;  // head_dim-64 kernel: warps 0-7 compute, 8-11 drain, 12 TMA, 13 MMA
-constexpr int kBwdThreads = 320;  // warps 0-7 compute (two warpgroups, 64 query columns each), warp 8 TMA, warp 9 MMA
-
-template <int D>
-struct BwdSmem {
-  static constexpr int kTile = 128 * D * 2;                       // 128 x D bf16
-  static constexpr int kStages = (D == 64) ? 2 : 1;               // Q + dO ring
-  static constexpr int kKOff = 0;
-  static constexpr int kVOff = kTile;
-  static constexpr int kQdOOff = 2 * kTile;                       // per stage: Q tile, dO tile
-  static constexpr int kDsOff = kQdOOff + kStages * 2 * kTile;    // dS^T as an MN-major operand: 2 x [128 x 128 B]
-  static constexpr int kStgOff = kDsOff + 32768;                  // fp32 staging: one [128 rows x 128 B] per warpgroup
-  static constexpr int kVecOff = kStgOff + 32768;                 // per stage: lse2[128], delta[128] fp32
-  // augmentation operands (K-major, no swizzle, 8-row groups 256 B apart): a constant [128 x 16] tile of ones and two
-  // [128 x 16] tiles with -lse2 / scale_log2 and -delta of the step's queries as bf16 high + low parts in columns 0 and 1
-  static constexpr int kOnesOff = kVecOff + kStages * 1024;       // 4 KB
-  static constexpr int kAugOff = kOnesOff + 4096;                 // 2 x 4 KB
-  static constexpr int kBarOff = kAugOff + 8192;
-  static constexpr int kTotal = kBarOff + 512 + 1024;
-};
+constexpr int kBwd64Threads = 448;   // warps 0-7 compute, 8-11 drain, 12 TMA, 13 MMA
+constexpr int kBwd128Threads = 768;  // 0-15 compute, 16-19 drain, 20 TMA, 21 and 22 MMA, 23 idle (registers are re-split per four warps)
 
 __global__ void flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                       const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ lse2,
@@ -92,318 +74,8 @@ __global__ void flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const
   }
 }
 
-__device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
-template <int D>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-flash_bwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_do,
-                 const __grid_constant__ CUtensorMap tmap_dqkv, const float* __restrict__ lse2, const float* __restrict__ delta,
-                 int S, int n_kv, int g, float scale, float scale_log2, int* __restrict__ status) {
-  using L = BwdSmem<D>;
-  constexpr int QS = L::kStages;
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* kv_full = bars;            // [1]
-  uint64_t* q_full = bars + 1;         // [QS]
-  uint64_t* q_empty = q_full + QS;     // [QS]
-  uint64_t* sdp_full = q_empty + QS;   // S^T and dP^T ready
-  uint64_t* pds_full = sdp_full + 1;   // P^T, dS^T written (one arrival per compute warp)
-  uint64_t* dq_full = pds_full + 1;    // dV, dK, dQ MMAs of this step finished
-  uint64_t* dq_drained = dq_full + 1;  // dQ read out of tensor memory (one arrival per warp)
-  uint64_t* aug_full = dq_drained + 1; // augmentation tiles of the step written (one arrival per compute warp)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aug_full + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int n_blk = S / 128;
-  const int n = n_blk - 1 - (int)blockIdx.x;   // key block; cheapest last
-  const int head = blockIdx.y;                  // kv-group-major query head index j*g + i
-  const int b = blockIdx.z;
-  const int j = head / g, i = head % g;
-  const int nq = n_kv * g;
-  const int q_col = (j * (g + 2) + i) * D, k_col = (j * (g + 2) + g) * D, v_col = k_col + D;
-  const int do_col = head * D;
-  const int grow0 = b * S;
-  const int steps = n_blk - n;                  // query blocks m = n .. n_blk-1
-  const float* lse2_h = lse2 + ((size_t)b * nq + head) * S;
-  const float* delta_h = delta + ((size_t)b * nq + head) * S;
-
-  if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    for (int s = 0; s < QS; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); }
-    mbar_init(sdp_full, 1);
-    mbar_init(pds_full, 8);        // one arrival per compute warp
-    mbar_init(dq_full, 1);
-    mbar_init(dq_drained, 8);
-    mbar_init(aug_full, 8);
-    *abort_flag = 0;
-    fence_barrier_init();
-    fence_proxy_async();
-  }
-  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  // columns: S^T/P^T [0,128)  dP^T/dS^T [128,256)  D=64: dQ [256,320) dK [320,384) dV [384,448)
-  //                                                 D=128: dK [256,384) dV [384,512), dQ reuses [0,128) once P^T is consumed
-  const uint32_t tm_s = tmem_base, tm_dp = tmem_base + 128;
-  const uint32_t tm_dq = (D == 64) ? tmem_base + 256 : tmem_base;
-  const uint32_t tm_dk = (D == 64) ? tmem_base + 320 : tmem_base + 256;
-  const uint32_t tm_dv = (D == 64) ? tmem_base + 384 : tmem_base + 384;
-  constexpr bool kDqAliasesS = (D != 64);
-
-  if (warp == 8) {
-    // ---------------- TMA producer ----------------
-    if (elect_one()) {
-      tma_prefetch_desc(&tmap_qkv);
-      tma_prefetch_desc(&tmap_do);
-      mbar_expect_tx(kv_full, 2 * L::kTile);
-      for (int c = 0; c < D / 64; ++c) {
-        tma_load_2d(smem + L::kKOff + c * 16384, &tmap_qkv, k_col + c * 64, grow0 + n * 128, kv_full);
-        tma_load_2d(smem + L::kVOff + c * 16384, &tmap_qkv, v_col + c * 64, grow0 + n * 128, kv_full);
-      }
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int st = 0; st < steps; ++st) {
-        const int m = n + st;
-        if (!mbar_wait(&q_empty[stage], phase ^ 1, abort_flag, status, kTimeoutSmemEmpty)) break;
-        unsigned char* sq = smem + L::kQdOOff + stage * 2 * L::kTile;
-        unsigned char* sdo = sq + L::kTile;
-        float* vec = reinterpret_cast<float*>(smem + L::kVecOff + stage * 1024);
-        mbar_expect_tx(&q_full[stage], 2 * L::kTile + 1024);
-        for (int c = 0; c < D / 64; ++c) {
-          tma_load_2d(sq + c * 16384, &tmap_qkv, q_col + c * 64, grow0 + m * 128, &q_full[stage]);
-          tma_load_2d(sdo + c * 16384, &tmap_do, do_col + c * 64, grow0 + m * 128, &q_full[stage]);
-        }
-        bulk_load_1d(vec, lse2_h + m * 128, 512, &q_full[stage]);
-        bulk_load_1d(vec + 128, delta_h + m * 128, 512, &q_full[stage]);
-        if (++stage == QS) { stage = 0; phase ^= 1; }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 9) {
-    // ---------------- MMA issuer ----------------
-    if (elect_one()) {
-      constexpr uint32_t idesc_st = make_idesc_bf16(128, 128, false, false);   // S^T, dP^T: both operands K-major
-      constexpr uint32_t idesc_dkv = make_idesc_bf16(128, D, false, true);     // A from TMEM, B MN-major
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, D, true, true);       // A = dS^T in smem (MN-major), B = K MN-major
-      const uint32_t k_addr = smem_u32(smem + L::kKOff), v_addr = smem_u32(smem + L::kVOff);
-      const uint32_t ds_addr = smem_u32(smem + L::kDsOff);
-      bool ok = mbar_wait(kv_full, 0, abort_flag, status, kTimeoutSmemFull);
-      int stage = 0;
-      uint32_t phase = 0, ph_pds = 0, ph_drain = 0, ph_aug = 0;
-      auto issue_sdp = [&](uint32_t q_addr, uint32_t do_addr) {
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk / 4) * 16384 + (kk % 4) * 32;
-          umma_bf16_ss(tm_s, make_smem_desc(k_addr + off, 0, 1024), make_smem_desc(q_addr + off, 0, 1024), idesc_st, kk != 0);
-        }
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk / 4) * 16384 + (kk % 4) * 32;
-          umma_bf16_ss(tm_dp, make_smem_desc(v_addr + off, 0, 1024), make_smem_desc(do_addr + off, 0, 1024), idesc_st, kk != 0);
-        }
-        // one more k-step each: ones x (-lse2 / scale_log2) and ones x (-delta), so the accumulators hold the exp2 argument
-        // and dP - delta and the compute warps fetch no per-query vectors (their broadcast shared-memory loads were what the
-        // math phase waited for)
-        const uint64_t ones_desc = make_smem_desc_plain(smem_u32(smem + L::kOnesOff), 128, 256);
-        umma_bf16_ss(tm_s, ones_desc, make_smem_desc_plain(smem_u32(smem + L::kAugOff), 128, 256), idesc_st, 1u);
-        umma_bf16_ss(tm_dp, ones_desc, make_smem_desc_plain(smem_u32(smem + L::kAugOff + 4096), 128, 256), idesc_st, 1u);
-        umma_commit(sdp_full);
-      };
-      if (ok) ok = mbar_wait(&q_full[0], 0, abort_flag, status, kTimeoutSmemFull);
-      if (ok) { ok = mbar_wait(aug_full, ph_aug, abort_flag, status, kTimeoutSmemFull); ph_aug ^= 1; }
-      if (ok) {
-        tc_fence_after();
-        const uint32_t q0a = smem_u32(smem + L::kQdOOff);
-        issue_sdp(q0a, q0a + L::kTile);
-      }
-      for (int st = 0; st < steps && ok; ++st) {
-        const uint32_t q_addr = smem_u32(smem + L::kQdOOff + stage * 2 * L::kTile);
-        const uint32_t do_addr = q_addr + L::kTile;
-        if (!mbar_wait(pds_full, ph_pds, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
-        ph_pds ^= 1;
-        tc_fence_after();
-        // dV += P^T dO ; dK += dS^T Q   (K dimension = 128 queries, 8 steps of 16)
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16_ts(tm_dv, tm_s + (kk < 4 ? kk * 8 : 64 + (kk - 4) * 8), make_smem_desc(do_addr + kk * 2048, 16384, 1024),
-                       idesc_dkv, (st | kk) != 0);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16_ts(tm_dk, tm_dp + (kk < 4 ? kk * 8 : 64 + (kk - 4) * 8), make_smem_desc(q_addr + kk * 2048, 16384, 1024),
-                       idesc_dkv, (st | kk) != 0);
-        // dQ = dS K : M = queries, N = D, K dimension = 128 keys
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16_ss(tm_dq, make_smem_desc(ds_addr + kk * 2048, 16384, 1024), make_smem_desc(k_addr + kk * 2048, 16384, 1024),
-                       idesc_dq, kk != 0);
-        umma_commit(dq_full);
-        umma_commit(&q_empty[stage]);
-        int nstage = stage + 1;
-        uint32_t nphase = phase;
-        if (nstage == QS) { nstage = 0; nphase ^= 1; }
-        if (st + 1 < steps) {
-          if (!mbar_wait(&q_full[nstage], nphase, abort_flag, status, kTimeoutSmemFull)) { ok = false; break; }
-          if (kDqAliasesS) {
-            if (!mbar_wait(dq_drained, ph_drain, abort_flag, status, kTimeoutTmemEmpty)) { ok = false; break; }
-            ph_drain ^= 1;
-          }
-          if (!mbar_wait(aug_full, ph_aug, abort_flag, status, kTimeoutSmemFull)) { ok = false; break; }
-          ph_aug ^= 1;
-          tc_fence_after();
-          const uint32_t qn = smem_u32(smem + L::kQdOOff + nstage * 2 * L::kTile);
-          issue_sdp(qn, qn + L::kTile);
-        }
-        stage = nstage;
-        phase = nphase;
-      }
-    }
-    __syncwarp();
-  } else {
-    // ---------------- compute warps ----------------
-    // Thread (qd, lane) owns key row r = 32*qd + lane; warpgroup h = warp / 4 owns query columns [64h, 64h+64).
-    const int qd = warp % 4, h = warp / 4;
-    const int r = qd * 32 + lane;
-    const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-    const int key = n * 128 + r;
-    unsigned char* ds_row = smem + L::kDsOff + h * 16384 + r * 128;   // dS^T operand chunk h (queries 64h..64h+63)
-    unsigned char* stg = smem + L::kStgOff + h * 16384;
-    const bool issuer = (threadIdx.x == h * 128);
-    const int bar_id = 1 + h;
-    uint32_t ph_sdp = 0, ph_dq = 0;
-    int stage = 0;
-    uint32_t qphase = 0;
-    bool ok = true;
-    // TMA reduce-add of this warpgroup's half of a [128 x D] fp32 tensor-memory tile into the fp32 dQKV image
-    auto drain_tile = [&](uint32_t tm_src, int col, int row) {
-#pragma unroll 1
-      for (int c = 0; c < D / 64; ++c) {
-        const int cc = h * (D / 64) + c;     // 32-column chunk index handled by this warpgroup
-        uint32_t v[32];
-        tmem_ld_32x32(tm_src + lane_off + cc * 32, v);
-        tmem_wait_ld();
-        if (issuer) tma_wait_group_read<0>();  // the previous store has finished reading the staging buffer
-        named_barrier_sync(bar_id, 128);
-        unsigned char* rowp = stg + r * 128;
-#pragma unroll
-        for (int p8 = 0; p8 < 8; ++p8)
-          *reinterpret_cast<uint4*>(rowp + ((p8 ^ (r & 7)) * 16)) = make_uint4(v[p8 * 4], v[p8 * 4 + 1], v[p8 * 4 + 2], v[p8 * 4 + 3]);
-        fence_proxy_async();
-        named_barrier_sync(bar_id, 128);
-        if (issuer) {
-          tma_reduce_add_2d(&tmap_dqkv, stg, col + cc * 32, row);
-          tma_commit_group();
-        }
-      }
-    };
-    {
-      // one-time: zero the augmentation tiles (only columns 0 and 1 are rewritten) and build the ones tile
-      const int t = threadIdx.x;   // 0 .. 255
-      uint4* z = reinterpret_cast<uint4*>(smem + L::kAugOff);
-      for (int i = t; i < 8192 / 16; i += 256) z[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (t < 128) {
-        unsigned char* one_row = smem + L::kOnesOff + (t >> 3) * 256 + (t & 7) * 16;
-        *reinterpret_cast<uint4*>(one_row) = make_uint4(0x3F803F80u, 0u, 0u, 0u);   // bf16 1.0, 1.0, zeros
-        *reinterpret_cast<uint4*>(one_row + 128) = make_uint4(0u, 0u, 0u, 0u);
-      }
-      named_barrier_sync(3, 256);
-    }
-    const float inv_scale_log2 = 1.f / scale_log2, inv_scale = 1.f / scale;
-    for (int st = 0; st < steps && ok; ++st) {
-      const int m = n + st;
-      // q_full is also what delivers lse2 / delta of this query block
-      if (!mbar_wait(&q_full[stage], qphase, abort_flag, status, kTimeoutSmemFull)) { ok = false; break; }
-      {
-        // thread t < 128 writes the S^T tile's row of query t, thread 128 + t the dP^T tile's: value as bf16 high + low part.
-        // The previous step's products have finished reading the tiles (this warp has seen their sdp_full).
-        const int t = threadIdx.x, q = t & 127;
-        const float* vsrc = reinterpret_cast<const float*>(smem + L::kVecOff + stage * 1024);
-        const float val = (t < 128) ? -vsrc[q] * inv_scale_log2 : -vsrc[128 + q] * inv_scale;
-        const __nv_bfloat16 hi = __float2bfloat16(val);
-        const __nv_bfloat16 lo = __float2bfloat16(val - __bfloat162float(hi));
-        unsigned char* dst = smem + L::kAugOff + (t < 128 ? 0 : 4096) + (q >> 3) * 256 + (q & 7) * 16;
-        *reinterpret_cast<uint32_t*>(dst) = (uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(lo) << 16);
-        fence_proxy_async();
-        mbar_arrive_warp(aug_full);
-      }
-      if (!mbar_wait(sdp_full, ph_sdp, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
-      ph_sdp ^= 1;
-      tc_fence_after();
-      const bool diag = (m == n);
-      uint32_t sv[64], dv[64];
-      tmem_ld_32x32(tm_s + lane_off + 64 * h, sv);
-      tmem_ld_32x32(tm_s + lane_off + 64 * h + 32, sv + 32);
-      tmem_ld_32x32(tm_dp + lane_off + 64 * h, dv);
-      tmem_ld_32x32(tm_dp + lane_off + 64 * h + 32, dv + 32);
-      tmem_wait_ld();
-      const int q_first = m * 128 + 64 * h;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t pk[16], dk[16];
-#pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          const int qc = c * 32 + e;
-          float p0 = exp2f(__uint_as_float(sv[qc]) * scale_log2);        // the accumulator already holds S - lse
-          float p1 = exp2f(__uint_as_float(sv[qc + 1]) * scale_log2);
-          if (diag) {
-            if (key > q_first + qc) p0 = 0.f;
-            if (key > q_first + qc + 1) p1 = 0.f;
-          }
-          const float d0 = (p0 * scale) * __uint_as_float(dv[qc]);           // ... and dP - delta
-          const float d1 = (p1 * scale) * __uint_as_float(dv[qc + 1]);
-          pk[e / 2] = pack_bf16(p0, p1);
-          dk[e / 2] = pack_bf16(d0, d1);
-        }
-        // P^T / dS^T of queries [64h+32c, +32) go to packed columns [64h+16c, +16): inside this warpgroup's own
-        // S^T / dP^T column range, all of which this thread has already read
-        tmem_st_32x16(tm_s + lane_off + 64 * h + c * 16, pk);
-        tmem_st_32x16(tm_dp + lane_off + 64 * h + c * 16, dk);
-#pragma unroll
-        for (int p4 = 0; p4 < 4; ++p4) {
-          const int piece = c * 4 + p4;
-          *reinterpret_cast<uint4*>(ds_row + ((piece ^ (r & 7)) * 16)) = make_uint4(dk[p4 * 4], dk[p4 * 4 + 1], dk[p4 * 4 + 2], dk[p4 * 4 + 3]);
-        }
-      }
-      tmem_wait_st();
-      fence_proxy_async();
-      tc_fence_before();
-      mbar_arrive_warp(pds_full);
-      // drain dQ of this step
-      if (!mbar_wait(dq_full, ph_dq, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
-      ph_dq ^= 1;
-      tc_fence_after();
-      drain_tile(tm_dq, q_col, grow0 + m * 128);
-      tc_fence_before();
-      mbar_arrive_warp(dq_drained);
-      if (++stage == QS) { stage = 0; qphase ^= 1; }
-    }
-    if (ok) {
-      // the last dq_full also covers the final dK / dV accumulation
-      drain_tile(tm_dk, k_col, grow0 + n * 128);
-      drain_tile(tm_dv, v_col, grow0 + n * 128);
-    }
-    if (issuer) tma_wait_group<0>();
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  if (*abort_flag) {
-    const long long t0 = clock64();
-    while (clock64() - t0 < 2000000LL) { __nanosleep(200); }
-    __syncthreads();
-  }
-  if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
-}
-
 // ---------------------------------------------------------------------------------------------------------------------
-// head_dim 64 backward, software-pipelined.  Same math and data flow as flash_bwd_kernel, but the 128-query block of a step
-// is handled as two 64-query halves with their own barriers, so the long serial chain of a step (commit -> tensor-memory
+// head_dim 64 backward, software-pipelined.  The 128-query block of a step is handled as two 64-query halves with their own barriers, so the long serial chain of a step (commit -> tensor-memory
 // load -> exp / dS math -> tensor-memory store -> fence -> barrier -> next MMA) of one half runs while the tensor core
 // works on the other half and on the next step:
 //     MMA order:  ... | dV_A dK_A (i) | S_A dP_A (i+1) | dV_B dK_B (i) | dQ (i) | S_B dP_B (i+1) | dV_A dK_A (i+1) | ...
@@ -772,6 +444,399 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
   if (warp == 13) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// head_dim 128 backward.  Same math, on a stream of 64-query half blocks k = 0, 1, ... of the CTA's 128-key block, so that the
+// tensor core never waits for the chain  S^T -> exp -> dP^T -> dS^T  of one half: it has the other half's products to run.
+//     products:  ... | dP(k+1) | dV(k) dK(k) | S(k+2), dQ(k) | dP(k+2) | dV(k+1) dK(k+1) | S(k+3), dQ(k+1) | ...
+// The compute warps of parity h own the halves of parity h: the exponentials of k + 1 run under the products of k - 1, its dS^T
+// under those of k.  Tensor memory (512 columns): S^T of two halves 128, dP^T 64, dQ^T 64, dK 128, dV 128.  P^T and dS^T of a
+// half share the columns of its S^T, so dP^T is free as soon as it has been read.
+// dQ is taken transposed, [128 d x 64 queries] = K^T dS^T: a 64-row accumulator would need twice the columns, and a warp that
+// owns 32 neighbouring d of a query adds its 128 bytes straight from registers into the fp32 image (red.global; a TMA
+// reduce-add through shared memory measured 3 % slower).
+// Bound: the tensor core, 1740 cycles a half (measured alone: 52 cycles a 128 x 64 SS product, 64 a 128 x 128 TS product), of which
+// about 60 % is reached.  1 x 4096 tokens, 32/2 heads: 659 us with one 128-query block at a time and every stage of it in
+// series -> 346 us = 0.60 of the measured 1668 TFLOP/s.
+// ---------------------------------------------------------------------------------------------------------------------
+struct Bwd128Smem {
+  static constexpr int kTile = 128 * 128 * 2;             // K, V: two 64-column chunks of 16 KB
+  static constexpr int kHalf = 64 * 128 * 2;              // 64 rows of Q or dO: two 64-column chunks of 8 KB
+  static constexpr int kQStages = 4, kDoStages = 3;
+  static constexpr int kKOff = 0;
+  static constexpr int kVOff = kTile;
+  static constexpr int kQOff = 2 * kTile;                 // after the last step: staging of dK (64 KB)
+  static constexpr int kDoOff = kQOff + kQStages * kHalf; // after the last step: staging of dV, with the first dS^T buffer
+  static constexpr int kDsOff = kDoOff + kDoStages * kHalf;  // two [128 keys x 64 queries] bf16
+  // k-step operands [rows x 16] (see flash_bwd64_kernel) of which only columns 0 and 1 are not zero: the first 16 bytes of the
+  // rows lie together (128 B per 8 rows), the second 16 bytes of every row are one block of zeros shared by all of them
+  static constexpr int kOnesOff = kDsOff + 2 * 16384;     // [128 x 16] with ones in columns 0, 1
+  static constexpr int kAugOff = kOnesOff + 2048;         // per Q stage [64 x 16] of -lse2 / scale_log2 and of -delta
+  static constexpr int kZeroOff = kAugOff + kQStages * 2048;
+  static constexpr int kBarOff = kZeroOff + 2048;
+  static constexpr int kTotal = kBarOff + 512 + 1024;
+};
+static_assert(Bwd128Smem::kTotal <= 232448, "shared memory per CTA");
+
+__device__ __forceinline__ void red_add_f32(float* p, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+
+// Register split of the 80 x 768 a launch gets: four compute warpgroups keep theirs, the drain warps take what the producer and
+// the issuers give up.
+constexpr int kBwd128RegsDrain = 104, kBwd128RegsMisc = 56;
+static_assert(4 * 80 + kBwd128RegsDrain + kBwd128RegsMisc <= 6 * 80, "more registers than the launch has");
+
+// The SS and TS products with operand descriptors given as words (low: address and leading offset; high: constant).
+__device__ __forceinline__ void umma_bf16_ss_words(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                                   uint32_t idesc, bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"((uint32_t)accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_ts_words(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                                   bool accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"((uint32_t)accumulate)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(kBwd128Threads, 1)
+flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_q64,
+                    const __grid_constant__ CUtensorMap tmap_do64, const __grid_constant__ CUtensorMap tmap_dqkv,
+                    float* __restrict__ img, const float* __restrict__ lse2, const float* __restrict__ delta, int S, int n_kv,
+                    int g, int heads_per_cta, float scale, float scale_log2, int* __restrict__ status) {
+  using L = Bwd128Smem;
+  constexpr int D = 128;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
+  uint64_t* kv_full = bars;                          // [1]
+  uint64_t* q_full = bars + 1;                       // [kQStages] Q and, with 4 arrivals, the augmentation rows of the half
+  uint64_t* q_empty = q_full + L::kQStages;          // [kQStages]
+  uint64_t* do_full = q_empty + L::kQStages;         // [kDoStages]
+  uint64_t* do_empty = do_full + L::kDoStages;       // [kDoStages]
+  uint64_t* s_full = do_empty + L::kDoStages;        // [2] by parity of the half
+  uint64_t* dp_full = s_full + 2;                    // [2] by parity
+  uint64_t* dp_read = dp_full + 2;                   // dP^T is in registers (8 arrivals)
+  uint64_t* pds_full = dp_read + 1;                  // [2] P^T, dS^T written (8 arrivals)
+  uint64_t* p_free = pds_full + 2;                   // [2] dV and dK of the half have read its P^T and dS^T
+  uint64_t* dq_full = p_free + 2;                    // [2] by parity
+  uint64_t* dq_drained = dq_full + 2;                // 4 arrivals
+  uint64_t* done = dq_drained + 1;                   // every product is finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int n_blk = S / 128, nq = n_kv * g;
+  // key block 0 has the most query blocks: the longest CTAs of a sequence start first, its one-step CTAs fill the tail
+  const int units = nq / heads_per_cta;
+  const int n = (int)blockIdx.x / units, head0 = (int)blockIdx.x % units * heads_per_cta, b = blockIdx.y;
+  const int j = head0 / g;                           // heads_per_cta divides g: one KV head per CTA
+  const int q_col0 = (j * (g + 2) + head0 % g) * D, k_col = (j * (g + 2) + g) * D, v_col = k_col + D;
+  const int grow0 = b * S;
+  const int steps = n_blk - n;                       // query blocks n .. n_blk-1 of a head
+  const int halves = 2 * steps * heads_per_cta;      // 64-query halves, the heads one after the other
+  const int row_first = n * 128;                     // sequence position of a head's first half
+
+  if (threadIdx.x == 0) {
+    mbar_init(kv_full, 1);
+    for (int s = 0; s < L::kQStages; ++s) { mbar_init(&q_full[s], 5); mbar_init(&q_empty[s], 1); }
+    for (int s = 0; s < L::kDoStages; ++s) { mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&s_full[s], 1); mbar_init(&dp_full[s], 1); mbar_init(&pds_full[s], 8);
+      mbar_init(&p_free[s], 1); mbar_init(&dq_full[s], 1);
+    }
+    mbar_init(dp_read, 8);
+    mbar_init(dq_drained, 4);
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  if (warp == 21) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tm_s = tmem_base, tm_dp = tmem_base + 128, tm_dq = tmem_base + 192, tm_dk = tmem_base + 256,
+                 tm_dv = tmem_base + 384;
+
+  if (warp >= 20) {
+    setmaxnreg_dec<kBwd128RegsMisc>();
+    if (warp == 20) {
+      // ---------------- TMA producer ----------------
+      if (elect_one()) {
+        tma_prefetch_desc(&tmap_qkv);
+        tma_prefetch_desc(&tmap_q64);
+        tma_prefetch_desc(&tmap_do64);
+        mbar_expect_tx(kv_full, 2 * L::kTile);
+        for (int c = 0; c < 2; ++c) {
+          tma_load_2d(smem + L::kKOff + c * 16384, &tmap_qkv, k_col + c * 64, grow0 + n * 128, kv_full);
+          tma_load_2d(smem + L::kVOff + c * 16384, &tmap_qkv, v_col + c * 64, grow0 + n * 128, kv_full);
+        }
+        int qs = 0, ds = 0;
+        uint32_t qph = 0, dph = 0;
+        int q_col = q_col0, do_col = head0 * D;
+        for (int k = 0, kh = 0; k < halves; ++k, ++kh) {
+          if (kh == 2 * steps) { kh = 0; q_col += D; do_col += D; }
+          const int row = grow0 + row_first + 64 * kh;
+          if (!mbar_wait(&q_empty[qs], qph ^ 1, abort_flag, status, kTimeoutSmemEmpty)) break;
+          mbar_expect_tx(&q_full[qs], L::kHalf);
+          for (int c = 0; c < 2; ++c)
+            tma_load_2d(smem + L::kQOff + qs * L::kHalf + c * 8192, &tmap_q64, q_col + c * 64, row, &q_full[qs]);
+          if (++qs == L::kQStages) { qs = 0; qph ^= 1; }
+          if (!mbar_wait(&do_empty[ds], dph ^ 1, abort_flag, status, kTimeoutSmemEmpty)) break;
+          mbar_expect_tx(&do_full[ds], L::kHalf);
+          for (int c = 0; c < 2; ++c)
+            tma_load_2d(smem + L::kDoOff + ds * L::kHalf + c * 8192, &tmap_do64, do_col + c * 64, row, &do_full[ds]);
+          if (++ds == L::kDoStages) { ds = 0; dph ^= 1; }
+        }
+      }
+      __syncwarp();
+    } else if (warp < 23) {
+      // ---------------- two MMA issuers: warp 21 S^T and dP^T, warp 22 dV, dK and dQ^T ----------------
+      // An issuer needs about 28 cycles a product and 100 a barrier poll: 2000 a half for one issuer, where the products need 1740
+      // by themselves.  Operand descriptors are a constant high word and a low word plus constants.
+      constexpr uint32_t kHi = (1024 >> 4) | (1u << 14) | (2u << 29);          // 8-row groups 1 KB apart, 128-byte swizzle
+      const uint32_t base = smem_u32(smem) >> 4;
+      const uint32_t k_lo = base + (L::kKOff >> 4), v_lo = base + (L::kVOff >> 4);
+      if (warp == 21 && elect_one()) {
+        constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, false, false);  // 128 keys x 64 queries
+        constexpr uint32_t kHiAug = (128 >> 4) | (1u << 14);                   // 8-row groups 128 B apart, no swizzle
+        const uint32_t ones_lo = (base + (L::kOnesOff >> 4)) | ((uint32_t)(L::kZeroOff - L::kOnesOff) << 12);
+        // x^T = A B^T for 64 queries, plus the k-step  ones x (-lse2 / scale_log2)  or  ones x (-delta)
+        auto issue_st = [&](uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t aug_off) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            umma_bf16_ss_words(d_tmem, a_lo + (((kk / 4) * 16384 + (kk % 4) * 32) >> 4), kHi,
+                               b_lo + (((kk / 4) * 8192 + (kk % 4) * 32) >> 4), kHi, idesc_st, kk != 0);
+          const uint32_t aug_lo = (base + (aug_off >> 4)) | ((L::kZeroOff - aug_off) << 12);
+          umma_bf16_ss_words(d_tmem, ones_lo, kHiAug, aug_lo, kHiAug, idesc_st, true);
+        };
+        auto do_s = [&](int k) -> bool {
+          const int st = k % L::kQStages;
+          if (!mbar_wait(&q_full[st], (k / L::kQStages) & 1, abort_flag, status, kTimeoutSmemFull)) return false;
+          tc_fence_after();
+          issue_st(tm_s + 64 * (k & 1), k_lo, base + ((L::kQOff + st * L::kHalf) >> 4), L::kAugOff + st * 2048);
+          umma_commit(&s_full[k & 1]);
+          return true;
+        };
+        int ds = 0;
+        uint32_t dph = 0;
+        auto do_dp = [&](int k) -> bool {
+          if (!mbar_wait(&do_full[ds], dph, abort_flag, status, kTimeoutSmemFull)) return false;
+          tc_fence_after();
+          issue_st(tm_dp, v_lo, base + ((L::kDoOff + ds * L::kHalf) >> 4), L::kAugOff + (k % L::kQStages) * 2048 + 1024);
+          umma_commit(&dp_full[k & 1]);
+          if (++ds == L::kDoStages) { ds = 0; dph ^= 1; }
+          return true;
+        };
+        bool ok = mbar_wait(kv_full, 0, abort_flag, status, kTimeoutSmemFull);
+        ok = ok && do_s(0) && do_s(1) && do_dp(0);
+        for (int k = 0; k + 1 < halves && ok; ++k) {
+          if (!mbar_wait(dp_read, k & 1, abort_flag, status, kTimeoutTmemEmpty)) break;
+          if (!do_dp(k + 1)) break;
+          if (k + 2 < halves) {
+            if (!mbar_wait(&p_free[k & 1], (k >> 1) & 1, abort_flag, status, kTimeoutTmemEmpty)) break;
+            if (!do_s(k + 2)) break;
+          }
+        }
+      }
+      if (warp == 22 && elect_one()) {
+        constexpr uint32_t idesc_dkv = make_idesc_bf16(128, D, false, true);   // A from tensor memory, B MN-major
+        constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64, true, true);    // A = K as [d x keys], B = dS^T, both MN-major
+        int ds = 0;
+        for (int k = 0; k < halves; ++k) {
+          const int par = k & 1, qs = k % L::kQStages;
+          if (!mbar_wait(&pds_full[par], (k >> 1) & 1, abort_flag, status, kTimeoutTmemFull)) break;
+          tc_fence_after();
+          // dV += P^T dO ; dK += dS^T Q  (64 queries = 4 steps of 16)
+          const uint32_t q_lo = (base + ((L::kQOff + qs * L::kHalf) >> 4)) | ((8192 >> 4) << 16);
+          const uint32_t do_lo = (base + ((L::kDoOff + ds * L::kHalf) >> 4)) | ((8192 >> 4) << 16);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            umma_bf16_ts_words(tm_dv, tm_s + 64 * par + (kk / 2) * 32 + (kk % 2) * 8, do_lo + ((kk * 2048) >> 4), kHi, idesc_dkv,
+                               kk != 0 || k != 0);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            umma_bf16_ts_words(tm_dk, tm_s + 64 * par + (kk / 2) * 32 + 16 + (kk % 2) * 8, q_lo + ((kk * 2048) >> 4), kHi, idesc_dkv,
+                               kk != 0 || k != 0);
+          umma_commit(&p_free[par]);
+          umma_commit(&q_empty[qs]);
+          umma_commit(&do_empty[ds]);
+          if (++ds == L::kDoStages) ds = 0;
+          if (k >= 1) {
+            if (!mbar_wait(dq_drained, par ^ 1, abort_flag, status, kTimeoutTmemEmpty)) break;
+            tc_fence_after();
+          }
+          const uint32_t ds_lo = (base + ((L::kDsOff + par * 16384) >> 4)) | ((16384 >> 4) << 16);
+          const uint32_t kt_lo = k_lo | ((16384 >> 4) << 16);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            umma_bf16_ss_words(tm_dq, kt_lo + ((kk * 2048) >> 4), kHi, ds_lo + ((kk * 2048) >> 4), kHi, idesc_dq, kk != 0);
+          umma_commit(&dq_full[par]);
+        }
+        umma_commit(done);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= 16) {
+    // ---------------- drain warps: dQ^T of every half into the fp32 image; augmentation rows ----------------
+    setmaxnreg_inc<kBwd128RegsDrain>();
+    const int qd = warp - 16, t = qd * 32 + lane;
+    const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
+    // thread t < 64 writes the S^T tile's row of query t, thread 64 + t the dP^T tile's: value as bf16 high + low part.
+    // The pre-pass stores delta * scale.  The rows are asked for in order: a head's halves are 64 apart, the next head's S later.
+    const float* aug_src = (t < 64 ? lse2 : delta) + ((size_t)b * nq + head0) * S + row_first + (t & 63);
+    int aug_k = 0;
+    auto next_aug = [&]() -> float {
+      const float val = *aug_src;
+      aug_src += 64;
+      if (++aug_k == 2 * steps) { aug_k = 0; aug_src += S - 128 * steps; }
+      return val;
+    };
+    const float aug_mul = t < 64 ? -1.f / scale_log2 : -1.f / scale;
+    auto write_aug = [&](int k, float raw) {
+      const float val = raw * aug_mul;
+      const __nv_bfloat16 hi = __float2bfloat16(val);
+      const __nv_bfloat16 lo = __float2bfloat16(val - __bfloat162float(hi));
+      const int st = k % L::kQStages;
+      *reinterpret_cast<uint32_t*>(smem + L::kAugOff + st * 2048 + t * 16) =
+          (uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(lo) << 16);
+      fence_proxy_async();
+      mbar_arrive_warp(&q_full[st]);
+    };
+    {
+      // one-time: zero the rows (only columns 0 and 1 are ever rewritten) and the shared zero block, and build the ones tile
+      uint4* z = reinterpret_cast<uint4*>(smem + L::kAugOff);
+      for (int e = t; e < (L::kBarOff - L::kAugOff) / 16; e += 128) z[e] = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(smem + L::kOnesOff + t * 16) = make_uint4(0x3F803F80u, 0u, 0u, 0u);   // bf16 1.0, 1.0, then zeros
+      named_barrier_sync(5, 128);
+      for (int k = 0; k < L::kQStages && k < halves; ++k) write_aug(k, next_aug());
+    }
+    // dq_full(k) means that S^T and dP^T of half k are done too, so the slot of half k can take half k + 4, whose S^T is two
+    // halves away.  The value is fetched one half ahead.
+    float vn = L::kQStages < halves ? next_aug() : 0.f;
+    const size_t rs = (size_t)n_kv * (g + 2) * D;
+    float* dst = img + (size_t)(grow0 + row_first) * rs + q_col0 + t;
+    for (int k = 0, kh = 0; k < halves; ++k, ++kh) {
+      if (kh == 2 * steps) { kh = 0; dst += D - (ptrdiff_t)(128 * steps) * (ptrdiff_t)rs; }
+      if (!mbar_wait(&dq_full[k & 1], (k >> 1) & 1, abort_flag, status, kTimeoutTmemFull)) break;
+      tc_fence_after();
+      uint32_t v[64];
+      tmem_ld_32x32(tm_dq + lane_off, v);
+      tmem_ld_32x32(tm_dq + lane_off + 32, v + 32);
+      tmem_wait_ld();
+      tc_fence_before();
+      mbar_arrive_warp(dq_drained);
+      if (k + 4 < halves) write_aug(k + 4, vn);
+      if (k + 5 < halves) vn = next_aug();
+#pragma unroll
+      for (int e = 0; e < 64; ++e) {
+        red_add_f32(dst, __uint_as_float(v[e]));
+        dst += rs;
+      }
+    }
+  } else {
+    // ---------------- compute warps ----------------
+    // Warpgroups 2h and 2h + 1 own the halves of parity h, 32 queries each; a thread owns one key row.  (One warpgroup per half,
+    // 64 queries a thread: its chain from S^T to dS^T, 2700 cycles, held the products up; 368 -> 346 us at the size above,
+    // together with two heads per CTA.)
+    const int qd = warp % 4, e = (warp / 4) % 2, h = warp / 8;
+    const int r = qd * 32 + lane;
+    const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
+    const uint32_t tm_sh = tm_s + 64 * h + 32 * e + lane_off, tm_dph = tm_dp + 32 * e + lane_off;
+    unsigned char* ds_row = smem + L::kDsOff + h * 16384 + r * 128;
+    bool ok = true;
+    for (int st = 0, sh = 0; 2 * st < halves; ++st, ++sh) {
+      if (sh == steps) sh = 0;
+      if (!mbar_wait(&s_full[h], st & 1, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
+      tc_fence_after();
+      // P^T lands on the first 16 of the warpgroup's 32 columns of S^T, dS^T on the others
+      float p[32];
+      {
+        uint32_t sv[32], pk[16];
+        tmem_ld_32x32(tm_sh, sv);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) p[c] = exp2f(__uint_as_float(sv[c]) * scale_log2);   // the accumulator holds S - lse
+        if (sh == 0) {   // the diagonal block
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            if (r > 64 * h + 32 * e + c) p[c] = 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c) pk[c] = pack_bf16(p[2 * c], p[2 * c + 1]);
+        tmem_st_32x16(tm_sh, pk);
+      }
+      if (!mbar_wait(&dp_full[h], st & 1, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
+      tc_fence_after();
+      {
+        // all of dP^T goes to registers at once: dP^T of the next half is issued as soon as it is out
+        uint32_t dv[32], dk[16];
+        tmem_ld_32x32(tm_dph, dv);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive_warp(dp_read);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const float d0 = (p[2 * c] * scale) * __uint_as_float(dv[2 * c]);                // dP - delta
+          const float d1 = (p[2 * c + 1] * scale) * __uint_as_float(dv[2 * c + 1]);
+          dk[c] = pack_bf16(d0, d1);
+        }
+        tmem_st_32x16(tm_sh + 16, dk);
+        // dQ^T of the last half of this parity has read the dS^T buffer
+        if (st > 0 && !mbar_wait(&dq_full[h], (st - 1) & 1, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
+#pragma unroll
+        for (int p4 = 0; p4 < 4; ++p4)
+          *reinterpret_cast<uint4*>(ds_row + (((4 * e + p4) ^ (r & 7)) * 16)) =
+              make_uint4(dk[p4 * 4], dk[p4 * 4 + 1], dk[p4 * 4 + 2], dk[p4 * 4 + 3]);
+      }
+      tmem_wait_st();
+      fence_proxy_async();
+      tc_fence_before();
+      mbar_arrive_warp(&pds_full[h]);
+    }
+    // warpgroups 0 and 1 hand on dK, 2 and 3 dV, 64 columns each: through the operand rings (every load has landed and been
+    // used) as [128 x 32] fp32 chunks of a TMA reduce-add
+    if (ok && mbar_wait(done, 0, abort_flag, status, kTimeoutTmemFull)) {
+      tc_fence_after();
+      unsigned char* stg = smem + (h == 0 ? L::kQOff : L::kDoOff) + e * 32768;
+#pragma unroll 1
+      for (int c = 0; c < 2; ++c) {
+        uint32_t v[32];
+        tmem_ld_32x32((h == 0 ? tm_dk : tm_dv) + lane_off + (2 * e + c) * 32, v);
+        tmem_wait_ld();
+        unsigned char* rowp = stg + c * 16384 + r * 128;
+#pragma unroll
+        for (int p8 = 0; p8 < 8; ++p8)
+          *reinterpret_cast<uint4*>(rowp + ((p8 ^ (r & 7)) * 16)) = make_uint4(v[p8 * 4], v[p8 * 4 + 1], v[p8 * 4 + 2], v[p8 * 4 + 3]);
+      }
+      fence_proxy_async();
+      named_barrier_sync(1 + warp / 4, 128);
+      if (r == 0) {
+        for (int c = 0; c < 2; ++c)
+          tma_reduce_add_2d(&tmap_dqkv, stg + c * 16384, (h == 0 ? k_col : v_col) + (2 * e + c) * 32, grow0 + n * 128);
+        tma_commit_group();
+        tma_wait_group<0>();
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) { __nanosleep(200); }
+    __syncthreads();
+  }
+  if (warp == 21) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+}
+
 // fp32 image -> bf16 packed dQKV.  With a RoPE table the inverse rotation (the RoPE backward) of the q and k head
 // slots is applied on the way, so the gradient needs no separate RoPE pass.
 __global__ void dqkv_finalize_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, const float* __restrict__ table,
@@ -804,6 +869,17 @@ __global__ void dqkv_finalize_kernel(const float* __restrict__ src, __nv_bfloat1
     store8(dst + off, x1);
     store8(dst + off + half, x2);
   }
+}
+
+// How many query heads of a KV group a head_dim-128 backward CTA walks.  More heads share one start (K and V tiles, filling the
+// pipeline) and one dK / dV hand-over, together about 2.5 steps (49 of 368 us at 1 x 4096 tokens, 32/2 heads, one head each); but a CTA of c * n_blk steps must not be long against an SM's share of
+// all steps, or the last ones to finish leave the others idle.
+static int bwd_heads_per_cta(int n_blk, int n_kv, int g, int B) {
+  const double share = (double)B * n_kv * g * n_blk * (n_blk + 1) / 2 / 148;
+  int best = 1;
+  for (int c = 2; c <= 4 && c <= g; ++c)
+    if (g % c == 0 && c * n_blk <= 0.6 * share) best = c;
+  return best;
 }
 
 int make_tmap_f32_2d(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
@@ -840,12 +916,10 @@ int fth_flash_bwd(const void* d_out, const void* qkv, const void* out, const flo
     flash_bwd_prep_kernel<<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, lse, delta, lse2,
                                                      B, S, nq, d, 1.f / sqrtf((float)d));
   }
-  CUtensorMap tq, tdo, tdq;
+  CUtensorMap tq, tdq;
   int r = make_tmap_bf16_2d(&tq, qkv, (uint64_t)B * S, rs, rs, 128, 64);
   if (r) return r;
-  r = make_tmap_bf16_2d(&tdo, d_out, (uint64_t)B * S, (uint64_t)nq * d, (uint64_t)nq * d, 128, 64);
-  if (r) return r;
-  CUtensorMap tq64, tdo64;   // 64-row boxes: the head_dim-64 kernel loads Q and dO per query half
+  CUtensorMap tq64, tdo64;   // 64-row boxes: Q and dO arrive per query half
   r = make_tmap_bf16_2d(&tq64, qkv, (uint64_t)B * S, rs, rs, 64, 64);
   if (r) return r;
   r = make_tmap_bf16_2d(&tdo64, d_out, (uint64_t)B * S, (uint64_t)nq * d, (uint64_t)nq * d, 64, 64);
@@ -861,9 +935,10 @@ int fth_flash_bwd(const void* d_out, const void* qkv, const void* out, const flo
                                                                         scale * 1.4426950408889634f, status, g_bwd_dbg);
   } else {
     static bool set = false;
-    if (!set) { cudaFuncSetAttribute(flash_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<128>::kTotal); set = true; }
-    flash_bwd_kernel<128><<<grid, kBwdThreads, BwdSmem<128>::kTotal, stream>>>(tq, tdo, tdq, lse2, delta, S, n_kv, g, scale,
-                                                                              scale * 1.4426950408889634f, status);
+    if (!set) { cudaFuncSetAttribute(flash_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::kTotal); set = true; }
+    const int hpc = bwd_heads_per_cta(S / 128, n_kv, g, B);
+    flash_bwd128_kernel<<<dim3(S / 128 * (nq / hpc), B), kBwd128Threads, Bwd128Smem::kTotal, stream>>>(
+        tq, tq64, tdo64, tdq, img, lse2, delta, S, n_kv, g, hpc, scale, scale * 1.4426950408889634f, status);
   }
   if (cudaGetLastError() != cudaSuccess) return -21;
   size_t items = (size_t)B * S * n_kv * (g + 2) * (d / 16);

@@ -235,6 +235,31 @@ def test_flash_fwd_work_items_and_growing_maxima(ops, B, S, nkv, g, d):
     assert float((lse - lse0).abs().max()) <= 1e-5 * float(lse0.abs().max()) + 1e-4
 
 
+@pytest.mark.parametrize("B,S,nkv,g", [(1, 128, 1, 1), (2, 256, 2, 3), (1, 384, 3, 5), (5, 1920, 4, 3), (4, 2048, 4, 4), (8, 1152, 8, 3), (16, 512, 8, 4)])
+def test_flash_bwd_d128_streams_of_halves(ops, B, S, nkv, g):
+    """The head_dim-128 backward on one key block (two halves: the rings never wrap), rings that wrap at every remainder, and
+    CTAs that walk one, two, three and four query heads of a KV group."""
+    from forge_train_harness_b200.ops.cuda_ops import check_status
+    d = 128
+    torch.manual_seed(S + g)
+    qkv = rnd(B * S, nkv * (g + 2) * d, scale=1.0)
+    dout = rnd(B * S, nkv * g * d, scale=1.0)
+    out, lse = ops.attention_fwd(qkv, S, nkv, g, d)
+    dqkv = ops.attention_bwd(dout, qkv, out, lse, S, nkv, g, d)
+    torch.cuda.synchronize()
+    check_status()
+    for b in range(B):   # one sequence at a time: the oracle keeps S x S scores
+        rows = slice(b * S, (b + 1) * S)
+        out0, lse0 = T.attention_fwd(qkv[rows].float(), S, nkv, g, d)
+        ref = T.attention_bwd(dout[rows].float(), qkv[rows].float(), out0, lse0, S, nkv, g, d).view(S, nkv, g + 2, d)
+        v = dqkv[rows].view(S, nkv, g + 2, d).float()
+        # P, dS, O and the result are each rounded to bf16 once (2^-9 of a value): four independent roundings of 2^-9 at most,
+        # every part by its own norm
+        for part in (slice(0, g), slice(g, g + 1), slice(g + 1, g + 2)):
+            err = (v[:, :, part] - ref[:, :, part]).norm() / ref[:, :, part].norm()
+            assert float(err) <= 4 * 2.0 ** -9, (b, part, float(err))
+
+
 def test_gemm_repeated_calls_and_views(ops):
     """Operands that are strided row views (unit inner stride) and repeated in-place updates."""
     big = rnd(512, 2048, scale=0.5)
