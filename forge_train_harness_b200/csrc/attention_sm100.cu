@@ -24,8 +24,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // Backward.
 //
 // Pre-pass (flash_bwd_prep_kernel): delta[b,h,s] = sum_d dO*O and lse2 = lse*log2(e), one warp per (row, head).
-// Main kernel: one CTA per (batch, query head, 128-key block n).  K and V tiles stay resident in shared memory; the CTA
-// walks the query blocks m >= n.  Per step, with every product on tcgen05 and every accumulator in tensor memory:
+// Main kernel: one CTA per (batch, 128-key block n, one to four query heads of a KV group).  K and V tiles stay resident; the CTA
+// walks the query blocks m >= n of its heads.  Per step, with every product on tcgen05 and every accumulator in tensor memory:
 //     S^T  = K Q^T          (128 keys x 128 queries)            SS-MMA
 //     dP^T = V dO^T                                              SS-MMA
 //     P^T  = exp2(S^T*c - lse2[q]),  dS^T = P^T (dP^T - delta[q]) * scale      (one thread per key row)
@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(kBwd64Threads, 1)
 flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_constant__ CUtensorMap tmap_q64,
                    const __grid_constant__ CUtensorMap tmap_do64,
                    const __grid_constant__ CUtensorMap tmap_dqkv, const float* __restrict__ lse2, const float* __restrict__ delta,
-                   int S, int n_kv, int g, float scale, float scale_log2, int* __restrict__ status, long long* __restrict__ dbg) {
+                   int S, int n_kv, int g, int heads_per_cta, float scale, float scale_log2, int* __restrict__ status,
+                   long long* __restrict__ dbg) {
   using L = Bwd64Smem;
   constexpr int D = 64;
   extern __shared__ unsigned char smem_raw[];
@@ -121,17 +122,15 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int n_blk = S / 128;
-  const int n = n_blk - 1 - (int)blockIdx.x;
-  const int head = blockIdx.y;
-  const int b = blockIdx.z;
-  const int j = head / g, i = head % g;
   const int nq = n_kv * g;
-  const int q_col = (j * (g + 2) + i) * D, k_col = (j * (g + 2) + g) * D, v_col = k_col + D;
-  const int do_col = head * D;
+  // key block 0 has the most query blocks: the longest CTAs of a sequence start first, its one-step CTAs fill the tail
+  const int units = nq / heads_per_cta;
+  const int n = (int)blockIdx.x / units, head0 = (int)blockIdx.x % units * heads_per_cta, b = blockIdx.y;
+  const int j = head0 / g;                      // heads_per_cta divides g: one KV head per CTA
+  const int q_col0 = (j * (g + 2) + head0 % g) * D, k_col = (j * (g + 2) + g) * D, v_col = k_col + D;
   const int grow0 = b * S;
-  const int steps = n_blk - n;
-  const float* lse2_h = lse2 + ((size_t)b * nq + head) * S;
-  const float* delta_h = delta + ((size_t)b * nq + head) * S;
+  const int steps_h = n_blk - n;                // query blocks n .. n_blk-1 of a head
+  const int steps = steps_h * heads_per_cta;    // the heads one after the other
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -169,10 +168,11 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
       // Q and dO arrive per query half: half h of a stage is free as soon as the dV / dK products of that half have
       // read it, half a step before the whole tile would be, which keeps the loads ahead of the shortened steps
       bool live = true;
-      for (int st = 0; st < steps && live; ++st) {
+      int q_col = q_col0, do_col = head0 * D;
+      for (int st = 0, m = n; st < steps && live; ++st, ++m) {
+        if (m == n_blk) { m = n; q_col += D; do_col += D; }
         const int stage = st & 1;
         const uint32_t phase = (st >> 1) & 1;
-        const int m = n + st;
         unsigned char* sq = smem + L::kQdOOff + stage * 2 * L::kTile;
         for (int h = 0; h < 2; ++h) {
           if (!mbar_wait(&q_empty[2 * stage + h], phase ^ 1, abort_flag, status, kTimeoutSmemEmpty)) { live = false; break; }
@@ -227,7 +227,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
       if (ok) { tc_fence_after(); issue_sdp(0, 0); }
       if (ok) ok = mbar_wait(&q_full[1], 0, abort_flag, status, kTimeoutSmemFull);
       if (ok) { tc_fence_after(); issue_sdp(0, 1); }
-      const bool mrec = dbg != nullptr && blockIdx.x == gridDim.x - 1 && blockIdx.y == 0 && blockIdx.z == 0;
+      const bool mrec = dbg != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
 #define FTH_MS(i) do { if (mrec && st < 64) dbg[(16 + (i)) * 64 + st] = clock64(); } while (0)
       for (int st = 0; st < steps && ok; ++st) {
         const int stage = st & 1, nstage = stage ^ 1;
@@ -310,8 +310,9 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
     // delta * scale) as bf16 hi + lo pairs in columns 0 and 1 of its row; the constant tile has ones in those two columns.
     const float inv_scale_log2 = 1.f / scale_log2, inv_scale = 1.f / scale;
     auto write_aug = [&](int st_for) {
-      const int m = n + st_for, hq = r >> 6, ql = r & 63;
-      const float vs = -lse2_h[m * 128 + r] * inv_scale_log2, vd = -delta_h[m * 128 + r] * inv_scale;
+      const int hd = st_for / steps_h, hq = r >> 6, ql = r & 63;
+      const size_t row = ((size_t)b * nq + head0 + hd) * S + (n + st_for - hd * steps_h) * 128 + r;
+      const float vs = -lse2[row] * inv_scale_log2, vd = -delta[row] * inv_scale;
       const __nv_bfloat16 s_hi = __float2bfloat16(vs), d_hi = __float2bfloat16(vd);
       const __nv_bfloat16 s_lo = __float2bfloat16(vs - __bfloat162float(s_hi)), d_lo = __float2bfloat16(vd - __bfloat162float(d_hi));
       unsigned char* base = smem + L::kAugOff + (st_for & 1) * 8192 + hq * 2048 + (ql >> 3) * 256 + (ql & 7) * 16;
@@ -350,14 +351,16 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
       tc_fence_before();
       mbar_arrive_warp(kv_tmem);
     }
-    for (int st = 0; st < steps && ok; ++st) {
+    int q_col = q_col0;
+    for (int st = 0, m = n; st < steps && ok; ++st, ++m) {
+      if (m == n_blk) { m = n; q_col += D; }
       if (!mbar_wait(&dq_full[0], st & 1, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
       tc_fence_after();
       // dq_full(st) also covers the S^T / dP^T products of step st + 1, so the tiles of parity st + 1 can take step st + 3
       // (and, the first time round, those of parity 0 step 2): always more than a step ahead of the MMA warp's need
       if (st == 0 && steps > 2) write_aug(2);
       if (st + 3 < steps) write_aug(st + 3);
-      drain64(tm_dq0, q_col, grow0 + (n + st) * 128, &dq_drained[0]);
+      drain64(tm_dq0, q_col, grow0 + m * 128, &dq_drained[0]);
     }
     if (ok) {   // the last dQ commit also covers the final dK / dV accumulation
       drain64(tm_dk, k_col, grow0 + n * 128, nullptr);
@@ -369,20 +372,18 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
     const int qd = warp % 4, h = warp / 4;
     const int r = qd * 32 + lane;
     const uint32_t lane_off = (uint32_t)(qd * 32) << 16;
-    const int key = n * 128 + r;
     bool ok = true;
-    const bool rec = dbg != nullptr && blockIdx.x == gridDim.x - 1 && blockIdx.y == 0 && blockIdx.z == 0 && qd == 0 && lane == 0;
+    const bool rec = dbg != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && qd == 0 && lane == 0;
     long long* drow = dbg + h * 8 * 64;
 #define FTH_TS(i) do { if (rec && st < 64) drow[(i) * 64 + st] = clock64(); } while (0)
-    for (int st = 0; st < steps && ok; ++st) {
-      const int m = n + st, stage = st & 1;
+    for (int st = 0, sh = 0; st < steps && ok; ++st, ++sh) {
+      if (sh == steps_h) sh = 0;
       FTH_TS(0);
       FTH_TS(6);
       if (!mbar_wait(&sdp_full[h], st & 1, abort_flag, status, kTimeoutTmemFull)) { ok = false; break; }
       FTH_TS(1);
       tc_fence_after();
-      const bool diag = (m == n);
-      const int q_first = m * 128 + 64 * h;
+      const bool diag = sh == 0;
       unsigned char* ds_row = smem + L::kDsOff + (st & 1) * 32768 + h * 16384 + r * 128;
       // Four 16-column chunks with a rolling prefetch: the tensor-memory load of chunk c+1 is in flight during the math
       // of chunk c.  The bf16 P^T / dS^T of chunk c land on columns [8c, 8c+8) of the warpgroup's own range, all of
@@ -407,7 +408,7 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_co
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               p[e] = exp2f(__uint_as_float(sv[c & 1][q4 * 4 + e]) * scale_log2);   // the accumulator already holds S - lse
-              if (kDiag) { if (key > q_first + c * 16 + q4 * 4 + e) p[e] = 0.f; }
+              if (kDiag) { if (r > 64 * h + c * 16 + q4 * 4 + e) p[e] = 0.f; }
               d[e] = (p[e] * scale) * __uint_as_float(dv[c & 1][q4 * 4 + e]);       // ... and dP - delta
             }
             pk[q4 * 2] = pack_bf16(p[0], p[1]); pk[q4 * 2 + 1] = pack_bf16(p[2], p[3]);
@@ -871,9 +872,10 @@ __global__ void dqkv_finalize_kernel(const float* __restrict__ src, __nv_bfloat1
   }
 }
 
-// How many query heads of a KV group a head_dim-128 backward CTA walks.  More heads share one start (K and V tiles, filling the
+// How many query heads of a KV group a backward CTA walks.  More heads share one start (K and V tiles, filling the
 // pipeline) and one dK / dV hand-over, together about 2.5 steps (49 of 368 us at 1 x 4096 tokens, 32/2 heads, one head each); but a CTA of c * n_blk steps must not be long against an SM's share of
 // all steps, or the last ones to finish leave the others idle.
+// head_dim 64, 4 x 4096 tokens, 16/2 heads: short CTAs first and one head each 465 us, long ones first and four heads each 421 us.
 static int bwd_heads_per_cta(int n_blk, int n_kv, int g, int B) {
   const double share = (double)B * n_kv * g * n_blk * (n_blk + 1) / 2 / 148;
   int best = 1;
@@ -927,17 +929,17 @@ int fth_flash_bwd(const void* d_out, const void* qkv, const void* out, const flo
   r = make_tmap_f32_2d(&tdq, img, (uint64_t)B * S, rs, rs, 128, 32);
   if (r) return r;
   const float scale = 1.f / sqrtf((float)d);
-  dim3 grid(S / 128, nq, B);
+  const int hpc = bwd_heads_per_cta(S / 128, n_kv, g, B);
+  const dim3 grid(S / 128 * (nq / hpc), B);
   if (d == 64) {
     static bool set = false;
     if (!set) { cudaFuncSetAttribute(flash_bwd64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd64Smem::kTotal); set = true; }
-    flash_bwd64_kernel<<<grid, kBwd64Threads, Bwd64Smem::kTotal, stream>>>(tq, tq64, tdo64, tdq, lse2, delta, S, n_kv, g, scale,
+    flash_bwd64_kernel<<<grid, kBwd64Threads, Bwd64Smem::kTotal, stream>>>(tq, tq64, tdo64, tdq, lse2, delta, S, n_kv, g, hpc, scale,
                                                                         scale * 1.4426950408889634f, status, g_bwd_dbg);
   } else {
     static bool set = false;
     if (!set) { cudaFuncSetAttribute(flash_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd128Smem::kTotal); set = true; }
-    const int hpc = bwd_heads_per_cta(S / 128, n_kv, g, B);
-    flash_bwd128_kernel<<<dim3(S / 128 * (nq / hpc), B), kBwd128Threads, Bwd128Smem::kTotal, stream>>>(
+    flash_bwd128_kernel<<<grid, kBwd128Threads, Bwd128Smem::kTotal, stream>>>(
         tq, tq64, tdo64, tdq, img, lse2, delta, S, n_kv, g, hpc, scale, scale * 1.4426950408889634f, status);
   }
   if (cudaGetLastError() != cudaSuccess) return -21;

@@ -235,12 +235,12 @@ def test_flash_fwd_work_items_and_growing_maxima(ops, B, S, nkv, g, d):
     assert float((lse - lse0).abs().max()) <= 1e-5 * float(lse0.abs().max()) + 1e-4
 
 
+@pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("B,S,nkv,g", [(1, 128, 1, 1), (2, 256, 2, 3), (1, 384, 3, 5), (5, 1920, 4, 3), (4, 2048, 4, 4), (8, 1152, 8, 3), (16, 512, 8, 4)])
-def test_flash_bwd_d128_streams_of_halves(ops, B, S, nkv, g):
-    """The head_dim-128 backward on one key block (two halves: the rings never wrap), rings that wrap at every remainder, and
-    CTAs that walk one, two, three and four query heads of a KV group."""
+def test_flash_bwd_streams_of_heads(ops, B, S, nkv, g, d):
+    """The backward on one key block (the rings never wrap), rings that wrap at every remainder, and CTAs that walk one, two,
+    three and four query heads of a KV group."""
     from forge_train_harness_b200.ops.cuda_ops import check_status
-    d = 128
     torch.manual_seed(S + g)
     qkv = rnd(B * S, nkv * (g + 2) * d, scale=1.0)
     dout = rnd(B * S, nkv * g * d, scale=1.0)
