@@ -94,6 +94,38 @@ def test_cross_entropy(ops, M, V):
     assert err < 4e-3, err
 
 
+@pytest.mark.parametrize("M,V", [(3, 5), (700, 4096), (600, 4099), (5, 8200), (4, 20480), (500, 20485), (4, 32768), (5, 32769), (3, 151940)])
+def test_cross_entropy_row_lengths(ops, M, V):
+    """Row lengths at the edges of the three forms of the kernel (registers, shared memory, read twice), ragged and whole last
+    vectors, more rows than resident CTAs, and targets of another shard; statistics and the fused gradient."""
+    from forge_train_harness_b200.ops.cuda_ops import _C
+    torch.manual_seed(V)
+    ld = (V + 7) // 8 * 8
+    logits = rnd(M, ld, scale=4.0)[:, :V]
+    labels = torch.randint(0, V, (M,), device="cuda", dtype=torch.int32)
+    labels[0], labels[-1] = V - 1, V + 3
+    mask = torch.ones(M, device="cuda")
+    mask[M // 2] = 0.0
+    lf = logits.double()
+    mx, sm, tg = _C.ce_stats(logits, labels, mask, 0)
+    has = labels < V
+    tg0 = torch.where(has, lf.gather(1, labels.clamp(max=V - 1).long()[:, None])[:, 0], torch.zeros_like(lf[:, 0]))
+    assert torch.equal(mx.double(), lf.max(dim=1).values) and torch.equal(tg.double(), tg0)
+    # fp32 exponentials (2^-21 or better each) and sums of at most 64 terms a thread, then a tree
+    sm0 = torch.exp(lf - mx.double()[:, None]).sum(dim=1)
+    assert float(((sm.double() - sm0) / sm0).abs().max()) < 1e-5
+    nll = ops.cross_entropy_fwd_bwd(logits, labels, mask, 0.25)
+    torch.cuda.synchronize()
+    lse = mx.double() + sm0.log()
+    assert float((nll.double() - (lse - tg0) * mask).abs().max()) < 1e-4
+    prob = torch.exp(lf - lse[:, None])
+    prob[has, labels[has].long()] -= 1.0
+    prob *= 0.25 * mask[:, None]
+    # one rounding to bf16 of a value whose exponent argument is fp32-accurate
+    assert float((logits.double() - prob).abs().max()) <= 2.0 ** -8 * 0.25
+    assert float((logits.double() - prob).norm() / prob.norm()) < 2.0 ** -8
+
+
 def test_ragged_vocab_shard_head(ops):
     """A vocabulary shard whose width is not a multiple of 8 (73448 / 4 = 18362): row-padded logits through the head GEMM,
     the fused cross-entropy statistics / gradient and the two backward GEMMs."""
